@@ -5,13 +5,25 @@
 // still-unvisited neighbours (descending index) and then stably sorts that run by
 // degree.  Hence, within one level,
 //   * child j belongs to the EARLIEST frontier position q adjacent to it
-//     (atomicMin over positions), and
+//     (atomicMin over positions),
 //   * the children of q are ordered by (degree ascending, index descending),
-//   * runs are concatenated in parent order (exclusive scan of run lengths).
-// Each level costs four kernels (claim, count, scan, write) plus a one-thread
-// advance kernel that also seeds the next connected component from the
-// caller's argsort(degree) order.  The host reads the level bounds back once per
-// level.
+//   * runs are concatenated in parent order (prefix sum of run lengths),
+// and a component starts at its first atom in the caller's argsort(degree) order.
+//
+// What bounds it is the chain of levels, not the edges (500,000 atoms in 60
+// components: 655 levels of about 760 atoms).  As five launches, a scan and two
+// copies to the host a level took 65 us, 43 ms in all.  So
+//   * all levels run in one cooperative kernel, one contiguous piece of the frontier
+//     a block, three grid barriers a level, its bounds kept on the device;
+//   * every component advances at once: components come from a union-find over the
+//     edges whose root is the component's earliest seed, the first frontier holds
+//     the roots in seed order, and a stable sort by component at the end puts the
+//     runs where the sequential order has them (12 levels instead of 655).
+// A directed adjacency (one that lists j under i and not i under j) may leave atoms
+// that their component's first seed does not reach; the same kernel then runs again
+// with one component at a time, each seeded when the frontier is empty.
+#include <algorithm>
+
 #include <cub/cub.cuh>
 
 #include "common.cuh"
@@ -19,125 +31,157 @@
 namespace inch {
 namespace {
 
-constexpr int kWarps = 8;
+constexpr int kWarps = 16;                  // warps of a BFS block
 constexpr int kCap = INCH_MAX_DEGREE;
+constexpr int kUnset = 0x7fffffff;
+constexpr int kTimeout = 8;
+constexpr unsigned kBarrierPolls = 1u << 24;   // bound of one grid barrier (seconds)
 
-struct State {
-  int64_t ls, le, n, seedptr;
+struct Ctl {
+  unsigned arrive;      // grid barrier
+  int bad;              // 1: seeds, 2: row length, 3: column (found before the BFS)
+  int flag;             // 4: more children than atoms, kTimeout: a barrier ran out
+  int levels;
+  int64_t visited;
+  int64_t seedptr;      // one component at a time: the next seed to look at
 };
 
-__global__ void k_init(int* __restrict__ pos, int* __restrict__ claim, int64_t n, State* st) {
+__global__ void k_check_seeds(const int64_t* __restrict__ seed_order, int64_t n, int* __restrict__ seen, Ctl* ctl) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    pos[i] = -1;
-    claim[i] = 0x7fffffff;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    st->ls = 0;
-    st->le = 0;
-    st->n = 0;
-    st->seedptr = 0;
+    int64_t s = seed_order[i];
+    if (s < 0 || s >= n || atomicAdd(&seen[s], 1) != 0) atomicExch(&ctl->bad, 1);
   }
 }
 
-// Frontier atom at position q claims every neighbour unvisited at level start.
-__global__ void k_claim(const int64_t* __restrict__ rowptr, const int* __restrict__ cols,
-                        const int* __restrict__ order, const int* __restrict__ pos, int* __restrict__ claim,
-                        const State* __restrict__ st) {
-  const int64_t ls = st->ls, le = st->le;
+// One warp per row (coalesced reads of the lists).
+__global__ void k_check_rows(const int64_t* __restrict__ rowptr, const int* __restrict__ cols, int64_t n, Ctl* ctl) {
   const int lane = threadIdx.x & 31;
-  for (int64_t q = ls + (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5); q < le;
-       q += (int64_t)gridDim.x * kWarps) {
-    int i = order[q];
-    for (int64_t e = rowptr[i] + lane; e < rowptr[i + 1]; e += 32) {
-      int j = cols[e];
-      if (pos[j] < 0) atomicMin(&claim[j], static_cast<int>(q));
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
+    const int64_t e0 = rowptr[i], d = rowptr[i + 1] - e0;
+    if (d < 0 || d > kCap) {
+      if (lane == 0) atomicExch(&ctl->bad, 2);
+      continue;
     }
+    bool out = false;
+    for (int64_t e = lane; e < d; e += 32) out |= cols[e0 + e] < 0 || cols[e0 + e] >= n;
+    if (out) atomicExch(&ctl->bad, 3);
   }
 }
 
-__global__ void k_count(const int64_t* __restrict__ rowptr, const int* __restrict__ cols,
-                        const int* __restrict__ order, const int* __restrict__ claim, int* __restrict__ cnt,
-                        const State* __restrict__ st) {
-  const int64_t ls = st->ls, le = st->le;
+__global__ void k_init(const int64_t* __restrict__ seed_order, int64_t n, int* __restrict__ order,
+                       int* __restrict__ claim, int* __restrict__ par, int* __restrict__ rank, const Ctl* ctl) {
+  if (ctl->bad) return;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    order[i] = -1;
+    claim[i] = kUnset;
+    par[i] = static_cast<int>(i);
+    rank[seed_order[i]] = static_cast<int>(i);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Components: union-find (Tarjan & van Leeuwen's path halving), parents always of
+// lower seed rank, so a root is its component's earliest seed whatever the order of
+// the unions.  Nothing waits: a failed exchange means that another union went ahead.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ int find_root(int* par, int x) {
+  int p = __ldcg(par + x);
+  while (p != x) {
+    const int g = __ldcg(par + p);
+    if (g == p) return p;
+    par[x] = g;                     // an ancestor of x; x is no root and never becomes one again
+    x = g;
+    p = __ldcg(par + x);
+  }
+  return x;
+}
+
+// Joins the components of root a and atom j; the root of both afterwards.
+__device__ __forceinline__ int join(int* par, const int* __restrict__ rank, int a, int j) {
+  int b = find_root(par, j);
+  while (a != b) {
+    int hi = a, lo = b;
+    if (rank[hi] < rank[lo]) {
+      hi = b;
+      lo = a;
+    }
+    const int old = atomicCAS(par + hi, hi, lo);
+    if (old == hi) return lo;
+    a = find_root(par, old);
+    b = lo;
+  }
+  return a;
+}
+
+// A thread per row joins it to its first and middle neighbour: after it most rows
+// hang in few trees, and the pass over all edges mostly compares two parents.
+__global__ void k_join_few(const int64_t* __restrict__ rowptr, const int* __restrict__ cols, int64_t n,
+                           const int* __restrict__ rank, int* par, const Ctl* ctl) {
+  if (ctl->bad) return;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t e0 = rowptr[i], d = rowptr[i + 1] - e0;
+    if (d == 0) continue;
+    int r = find_root(par, static_cast<int>(i));
+    r = join(par, rank, r, cols[e0]);
+    join(par, rank, r, cols[e0 + d / 2]);
+  }
+}
+
+__global__ void k_join_all(const int64_t* __restrict__ rowptr, const int* __restrict__ cols, int64_t n,
+                           const int* __restrict__ rank, int* par, const Ctl* ctl) {
+  if (ctl->bad) return;
   const int lane = threadIdx.x & 31;
-  for (int64_t q = ls + (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5); q < le;
-       q += (int64_t)gridDim.x * kWarps) {
-    int i = order[q];
-    int c = 0;
-    for (int64_t e = rowptr[i] + lane; e < rowptr[i + 1]; e += 32) c += claim[cols[e]] == static_cast<int>(q);
-    c = warp_sum(c);
-    if (lane == 0) cnt[q - ls] = c;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
+    const int64_t e1 = rowptr[i + 1];
+    int r = find_root(par, static_cast<int>(i));
+#pragma unroll 4
+    for (int64_t e = rowptr[i] + lane; e < e1; e += 32) {
+      const int j = cols[e];
+      if (__ldcg(par + j) != r) r = join(par, rank, find_root(par, r), j);
+    }
   }
 }
 
-// Writes the children of q, ordered by (degree asc, index desc), after the level.
-__global__ void __launch_bounds__(kWarps * 32)
-k_write(const int64_t* __restrict__ rowptr, const int* __restrict__ cols, const int* __restrict__ degree,
-        int* __restrict__ order, int* __restrict__ pos, const int* __restrict__ claim,
-        const int* __restrict__ off, const State* __restrict__ st, int64_t n_atoms, int* __restrict__ flag) {
-  __shared__ int buf[kWarps][kCap];
-  const int64_t ls = st->ls, le = st->le;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int* s = buf[w];
-  for (int64_t q = ls + (int64_t)blockIdx.x * kWarps + w; q < le; q += (int64_t)gridDim.x * kWarps) {
-    int i = order[q];
-    int m = 0;
-    for (int64_t e0 = rowptr[i]; e0 < rowptr[i + 1]; e0 += 32) {
-      int64_t e = e0 + lane;
-      bool ok = false;
-      int j = 0;
-      if (e < rowptr[i + 1]) {
-        j = cols[e];
-        ok = claim[j] == static_cast<int>(q);
-      }
-      unsigned b = __ballot_sync(0xffffffffu, ok);
-      if (ok) s[m + __popc(b & ((1u << lane) - 1u))] = j;   // m + rank < degree(i) <= kCap
-      m += __popc(b);
+__global__ void k_flatten(int64_t n, int* par, const Ctl* ctl) {
+  if (ctl->bad) return;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    // read-only walk: a halving store here could put an inner node over a finished root
+    int x = static_cast<int>(i), p = __ldcg(par + x);
+    while (p != x) {
+      x = p;
+      p = __ldcg(par + x);
     }
-    __syncwarp();
-    const int64_t base = le + off[q - ls];
-    for (int t = lane; t < m; t += 32) {
-      int jt = s[t];
-      int dt = degree[jt];
-      int rank = 0;
-      for (int u = 0; u < m; ++u) {
-        int ju = s[u];
-        int du = degree[ju];
-        rank += (du < dt) || (du == dt && ju > jt);
-      }
-      if (base + rank < n_atoms) {
-        order[base + rank] = jt;
-        pos[jt] = static_cast<int>(base + rank);
-      } else {
-        atomicExch(flag, 4);
-      }
-    }
-    __syncwarp();
+    par[i] = x;
   }
 }
 
-// Closes the level and, when the frontier is empty, seeds the next component.
-__global__ void k_advance(int* __restrict__ order, int* __restrict__ pos, const int* __restrict__ off,
-                          const int64_t* __restrict__ seed_order, int64_t n_atoms, State* st) {
-  int64_t L = st->le - st->ls;
-  int64_t added = L > 0 ? off[L] : 0;
-  int64_t n = st->n + added;
-  st->ls = st->le;
-  st->le = n;
-  st->n = n;
-  if (st->ls == st->le && n < n_atoms) {
-    int64_t p = st->seedptr;
-    while (p < n_atoms && pos[seed_order[p]] >= 0) ++p;
-    if (p < n_atoms) {
-      int s = static_cast<int>(seed_order[p]);
-      order[n] = s;
-      pos[s] = static_cast<int>(n);
-      st->ls = n;
-      st->le = n + 1;
-      st->n = n + 1;
-      st->seedptr = p + 1;
+// root[r] = 1 where the r-th seed is a root (root[n] = 0): its prefix sum numbers
+// the components in seed order.
+__global__ void k_roots(const int64_t* __restrict__ seed_order, int64_t n, const int* __restrict__ par,
+                        int* __restrict__ root, const Ctl* ctl) {
+  const bool bad = ctl->bad != 0;
+  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r <= n; r += (int64_t)gridDim.x * blockDim.x)
+    root[r] = !bad && r < n && par[seed_order[r]] == static_cast<int>(seed_order[r]);
+}
+
+__global__ void k_seed(const int64_t* __restrict__ seed_order, int64_t n, const int* __restrict__ cidx,
+                       int* __restrict__ order, int* __restrict__ claim, const Ctl* ctl) {
+  if (ctl->bad) return;
+  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
+    if (cidx[r + 1] != cidx[r]) {
+      const int s = static_cast<int>(seed_order[r]);
+      order[cidx[r]] = s;
+      claim[s] = -1;
     }
-  }
+}
+
+// Component of the atom at each BFS position, the key of the last sort.
+__global__ void k_keys(const int* __restrict__ order, int64_t n, const int* __restrict__ par,
+                       const int* __restrict__ rank, const int* __restrict__ cidx, int* __restrict__ key) {
+  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x)
+    key[p] = cidx[rank[par[order[p]]]];
 }
 
 __global__ void k_finish(const int* __restrict__ order, int64_t n, int64_t* __restrict__ rcm,
@@ -149,51 +193,228 @@ __global__ void k_finish(const int* __restrict__ order, int64_t n, int64_t* __re
   }
 }
 
-__global__ void k_check_seeds(const int64_t* __restrict__ seed_order, int64_t n, int* __restrict__ seen,
-                              int* __restrict__ bad) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t s = seed_order[i];
-    if (s < 0 || s >= n || atomicAdd(&seen[s], 1) != 0) atomicExch(bad, 1);
+// ---------------------------------------------------------------------------
+// The BFS
+// ---------------------------------------------------------------------------
+// Grid barrier of a cooperative launch (every block resident).  The wait is bounded:
+// a block whose wait runs out records it and leaves, and so do the others.
+__device__ bool grid_barrier(Ctl* ctl, unsigned& target) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    target += gridDim.x;
+    __threadfence();
+    atomicAdd(&ctl->arrive, 1u);
+    int ok = 1;
+    const volatile unsigned* at = &ctl->arrive;
+    for (unsigned polls = 0; static_cast<int>(*at - target) < 0; ++polls)
+      if (polls > kBarrierPolls || ((polls & 1023) == 1023 && *(volatile int*)&ctl->flag == kTimeout)) {
+        atomicExch(&ctl->flag, kTimeout);
+        ok = 0;
+        break;
+      }
+    __threadfence();
+    s_ok = ok;
   }
+  __syncthreads();
+  return s_ok != 0;
 }
 
-__global__ void k_check_degree(const int64_t* __restrict__ rowptr, const int* __restrict__ cols,
-                               const int* __restrict__ degree, int64_t n, int* __restrict__ bad) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t d = rowptr[i + 1] - rowptr[i];
-    if (d < 0 || d > kCap) atomicExch(bad, 2);
-    for (int64_t e = rowptr[i]; e < rowptr[i + 1] && d >= 0 && d <= kCap; ++e)
-      if (cols[e] < 0 || cols[e] >= n) atomicExch(bad, 3);
+// Everything that another block writes during the kernel is read past L1 (__ldcg).
+// `comp` (n_comp at comp_count): all components at once; else one at a time.
+__global__ void __launch_bounds__(kWarps * 32, 2)
+k_bfs(const int64_t* __restrict__ rowptr, const int* __restrict__ cols, const int* __restrict__ degree,
+      const int64_t* __restrict__ seed_order, const int* __restrict__ par, const int* __restrict__ comp_count,
+      int64_t n, int* order, int* claim, int* cnt, int* blocksum, Ctl* ctl, int all) {
+  extern __shared__ int s_buf[];            // kCap per warp
+  __shared__ int64_t s_pre[kWarps], s_tot[kWarps];
+  if (ctl->bad) return;                     // set by earlier kernels only: the same for every block
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int* s = s_buf + w * kCap;
+  unsigned target = 0;
+  int64_t ls = 0, le = all ? *comp_count : 0;
+  int levels = 0;
+  for (;;) {
+    if (ls == le) {
+      if (all || le >= n) break;
+      // the first seed that no earlier component reached
+      if (blockIdx.x == 0 && w == 0) {
+        int64_t p = ctl->seedptr;
+        for (; p < n; p += 32) {
+          const bool open = p + lane < n && __ldcg(claim + seed_order[p + lane]) == kUnset;
+          const unsigned b = __ballot_sync(0xffffffffu, open);
+          if (b != 0) {
+            p += __ffs(b) - 1;
+            break;
+          }
+        }
+        if (lane == 0 && p < n) {
+          const int sd = static_cast<int>(seed_order[p]);
+          order[le] = sd;
+          claim[sd] = -1;
+          ctl->seedptr = p + 1;
+        }
+      }
+      if (!grid_barrier(ctl, target)) break;
+      le = ls + 1;
+    }
+    const int64_t L = le - ls;
+    const int64_t per = (L + gridDim.x - 1) / gridDim.x;
+    const int64_t q0 = min(ls + (int64_t)blockIdx.x * per, le), q1 = min(q0 + per, le);
+    // claim: an atom visited before this level carries a smaller position than any q
+    for (int64_t q = q0 + w; q < q1; q += kWarps) {
+      const int i = __ldcg(order + q);
+      if (i < 0) continue;                  // duplicated entries left a hole: refused below
+      const int64_t e1 = rowptr[i + 1];
+#pragma unroll 4
+      for (int64_t e = rowptr[i] + lane; e < e1; e += 32) {
+        const int j = cols[e];
+        if (__ldcg(claim + j) > static_cast<int>(q)) atomicMin(claim + j, static_cast<int>(q));
+      }
+    }
+    if (!grid_barrier(ctl, target)) break;
+    // count the children of each q, prefix sums within the block's piece
+    for (int64_t q = q0 + w; q < q1; q += kWarps) {
+      const int i = __ldcg(order + q);
+      int c = 0;
+      if (i >= 0) {
+        const int64_t e1 = rowptr[i + 1];
+#pragma unroll 4
+        for (int64_t e = rowptr[i] + lane; e < e1; e += 32) c += __ldcg(claim + cols[e]) == static_cast<int>(q);
+        c = warp_sum(c);
+      } else if (lane == 0) {
+        atomicExch(&ctl->flag, 4);          // a hole: some row lists an atom twice
+      }
+      if (lane == 0) {
+        cnt[q] = c;
+        if (q == ls) {
+          ++levels;
+        } else if (all && i >= 0) {
+          const int h = __ldcg(order + q - 1);
+          levels += h >= 0 && par[h] != par[i];   // a level of every component in the frontier
+        }
+      }
+    }
+    __syncthreads();
+    if (w == 0) {
+      int run = 0;
+      for (int64_t q = q0; q < q1; q += 32) {
+        const int v = q + lane < q1 ? cnt[q + lane] : 0;
+        int x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, x, o);
+          if (lane >= o) x += y;
+        }
+        if (q + lane < q1) cnt[q + lane] = run + x - v;
+        run += __shfl_sync(0xffffffffu, x, 31);
+      }
+      if (lane == 0) blocksum[blockIdx.x] = run;
+    }
+    if (!grid_barrier(ctl, target)) break;
+    int64_t pre = 0, tot = 0;
+    for (int b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
+      const int v = __ldcg(blocksum + b);
+      tot += v;
+      pre += b < blockIdx.x ? v : 0;
+    }
+    pre = warp_sum(pre);
+    tot = warp_sum(tot);
+    if (lane == 0) {
+      s_pre[w] = pre;
+      s_tot[w] = tot;
+    }
+    __syncthreads();
+    pre = tot = 0;
+#pragma unroll
+    for (int k = 0; k < kWarps; ++k) {
+      pre += s_pre[k];
+      tot += s_tot[k];
+    }
+    // write the children of q, ordered by (degree asc, index desc), after the level
+    for (int64_t q = q0 + w; q < q1; q += kWarps) {
+      const int i = __ldcg(order + q);
+      if (i < 0) continue;
+      const int64_t e1 = rowptr[i + 1];
+      int m = 0;
+#pragma unroll 4
+      for (int64_t e0 = rowptr[i]; e0 < e1; e0 += 32) {
+        const int64_t e = e0 + lane;
+        const int j = e < e1 ? cols[e] : 0;
+        const bool ok = e < e1 && __ldcg(claim + j) == static_cast<int>(q);
+        const unsigned b = __ballot_sync(0xffffffffu, ok);
+        if (ok) s[m + __popc(b & ((1u << lane) - 1u))] = j;   // m + rank < row length <= kCap
+        m += __popc(b);
+      }
+      __syncwarp();
+      const bool both = 2 * m <= kCap;      // degrees beside the indices
+      if (both)
+        for (int t = lane; t < m; t += 32) s[m + t] = degree[s[t]];
+      __syncwarp();
+      const int64_t base = le + pre + cnt[q];
+      for (int t = lane; t < m; t += 32) {
+        const int jt = s[t];
+        const int dt = both ? s[m + t] : degree[jt];
+        int rank = 0;
+        for (int u = 0; u < m; ++u) {
+          const int ju = s[u];
+          const int du = both ? s[m + u] : degree[ju];
+          rank += (du < dt) || (du == dt && ju > jt);
+        }
+        if (base + rank < n) order[base + rank] = jt;
+        else atomicExch(&ctl->flag, 4);
+      }
+      __syncwarp();
+    }
+    ls = le;
+    le += tot;
+    if (le > n) break;                      // the same in every block
+    if (!grid_barrier(ctl, target)) break;
   }
+  levels = warp_sum(levels);                // lane 0 of each warp counted
+  if (lane == 0 && levels != 0) atomicAdd(&ctl->levels, levels);
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctl->visited = le;
 }
 
 struct RcmWs {
-  int *pos, *claim, *order, *cnt, *off, *flag;
-  State* st;
+  int *order, *claim, *par, *rank, *cidx, *cnt, *key, *order2, *blocksum;
+  Ctl* ctl;
   void* cub_tmp;
   size_t cub_bytes;
 };
 
+constexpr int kMaxBlocks = 1024;            // blocks of the BFS kernel, at most
+
+size_t cub_bytes_for(int64_t n) {
+  size_t a = 0, b = 0;
+  cub::DeviceScan::ExclusiveSum(nullptr, a, (int*)nullptr, (int*)nullptr, (int)(n + 1));
+  cub::DeviceRadixSort::SortPairs(nullptr, b, (const int*)nullptr, (int*)nullptr, (const int*)nullptr, (int*)nullptr,
+                                  (int)n);
+  return a > b ? a : b;
+}
+
 template <class C>
 void carve_rcm(C& c, int64_t n, RcmWs* w) {
-  size_t cb = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, cb, (int*)nullptr, (int*)nullptr, (int)(n + 1));
+  const size_t cb = cub_bytes_for(n);
   if constexpr (std::is_same<C, Carver>::value) {
-    w->pos = c.template take<int>(n);
-    w->claim = c.template take<int>(n);
     w->order = c.template take<int>(n);
+    w->claim = c.template take<int>(n);
+    w->par = c.template take<int>(n);
+    w->rank = c.template take<int>(n);
+    w->cidx = c.template take<int>(n + 1);
     w->cnt = c.template take<int>(n + 1);
-    w->off = c.template take<int>(n + 1);
-    w->flag = c.template take<int>(4);
-    w->st = c.template take<State>(1);
+    w->key = c.template take<int>(n);
+    w->order2 = c.template take<int>(n);
+    w->blocksum = c.template take<int>(kMaxBlocks);
+    w->ctl = c.template take<Ctl>(1);
     w->cub_tmp = c.template take<char>(cb);
     w->cub_bytes = cb;
   } else {
-    for (int k = 0; k < 3; ++k) c.template take<int>(n);
-    c.template take<int>(n + 1);
-    c.template take<int>(n + 1);
-    c.template take<int>(4);
-    c.template take<State>(1);
+    for (int k = 0; k < 4; ++k) c.template take<int>(n);
+    for (int k = 0; k < 2; ++k) c.template take<int>(n + 1);
+    for (int k = 0; k < 2; ++k) c.template take<int>(n);
+    c.template take<int>(kMaxBlocks);
+    c.template take<Ctl>(1);
     c.template take<char>(cb);
   }
 }
@@ -221,56 +442,84 @@ extern "C" inch_status inch_rcm(const int64_t* rowptr, const int32_t* cols, cons
   RcmWs w;
   carve_rcm(c, n, &w);
   INCH_REQUIRE(c.ok, INCH_OOM, "inch_rcm: workspace of %zu bytes, need %zu", ws_bytes, inch_rcm_workspace_size(n));
-  const int bl = grid_for(n, 256, 148 * 16);
-  // Validate the inputs that index memory: seed_order must be a permutation,
-  // rows at most kCap long with in-range columns.
-  INCH_CUDA(cudaMemsetAsync(w.flag, 0, sizeof(int) * 4, stream));
-  INCH_CUDA(cudaMemsetAsync(w.pos, 0, sizeof(int) * n, stream));
-  k_check_seeds<<<bl, 256, 0, stream>>>(seed_order, n, w.pos, w.flag);
-  INCH_LAUNCH_CHECK();
-  k_check_degree<<<bl, 256, 0, stream>>>(rowptr, cols, degree, n, w.flag);
-  INCH_LAUNCH_CHECK();
-  int bad = 0;
-  INCH_CUDA(cudaMemcpyAsync(&bad, w.flag, sizeof(int), cudaMemcpyDeviceToHost, stream));
-  INCH_CUDA(cudaStreamSynchronize(stream));
-  INCH_REQUIRE(bad != 1, INCH_INVALID_ARG, "inch_rcm: seed_order is not a permutation of 0..n-1");
-  INCH_REQUIRE(bad != 2, INCH_LIMIT, "inch_rcm: a row has more than %d neighbours", kCap);
-  INCH_REQUIRE(bad == 0, INCH_INVALID_ARG, "inch_rcm: column index out of range");
+  constexpr int kSmem = kWarps * kCap * (int)sizeof(int);
+  int dev = 0, sms = 0, per_sm = 0;
+  INCH_CUDA(cudaGetDevice(&dev));
+  INCH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  INCH_CUDA(cudaFuncSetAttribute(k_bfs, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  INCH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bfs, kWarps * 32, kSmem));
+  INCH_REQUIRE(per_sm >= 1, INCH_CUDA_ERROR, "inch_rcm: the BFS kernel does not fit on an SM");
+  // one block per SM while a block's piece of all atoms is short (fewer blocks to
+  // wait for at a barrier), two where the frontiers are wide
+  const int64_t want = n > 200000 ? 2 : 1;
+  const int blocks = static_cast<int>(std::min<int64_t>(std::min<int64_t>(want, per_sm) * sms, kMaxBlocks));
+  const int bl = grid_for(n, 256, 148 * 16), bw = grid_for(n, 8, 148 * 16);
 
-  k_init<<<bl, 256, 0, stream>>>(w.pos, w.claim, n, w.st);
+  INCH_CUDA(cudaMemsetAsync(w.ctl, 0, sizeof(Ctl), stream));
+  INCH_CUDA(cudaMemsetAsync(w.cnt, 0, sizeof(int) * n, stream));
+  // Validate the inputs that index memory: seed_order must be a permutation, rows at
+  // most kCap long with in-range columns.  The kernels that follow do nothing where
+  // they are not.
+  k_check_seeds<<<bl, 256, 0, stream>>>(seed_order, n, w.cnt, w.ctl);
   INCH_LAUNCH_CHECK();
-  k_advance<<<1, 1, 0, stream>>>(w.order, w.pos, w.off, seed_order, n, w.st);
+  k_check_rows<<<bw, 256, 0, stream>>>(rowptr, cols, n, w.ctl);
   INCH_LAUNCH_CHECK();
-  State h{};
-  INCH_CUDA(cudaMemcpyAsync(&h, w.st, sizeof(State), cudaMemcpyDeviceToHost, stream));
-  INCH_CUDA(cudaStreamSynchronize(stream));
-  int levels = 0;
-  while (h.ls < h.le) {
-    const int64_t L = h.le - h.ls;
-    const int gw = grid_for(L, kWarps, 148 * 8);
-    k_claim<<<gw, kWarps * 32, 0, stream>>>(rowptr, cols, w.order, w.pos, w.claim, w.st);
-    INCH_LAUNCH_CHECK();
-    k_count<<<gw, kWarps * 32, 0, stream>>>(rowptr, cols, w.order, w.claim, w.cnt, w.st);
-    INCH_LAUNCH_CHECK();
-    INCH_CUDA(cudaMemsetAsync(w.cnt + L, 0, sizeof(int), stream));
-    size_t cb = w.cub_bytes;
-    INCH_CUDA(cub::DeviceScan::ExclusiveSum(w.cub_tmp, cb, w.cnt, w.off, (int)(L + 1), stream));
-    k_write<<<gw, kWarps * 32, 0, stream>>>(rowptr, cols, degree, w.order, w.pos, w.claim, w.off, w.st, n,
-                                           w.flag);
-    INCH_LAUNCH_CHECK();
-    k_advance<<<1, 1, 0, stream>>>(w.order, w.pos, w.off, seed_order, n, w.st);
-    INCH_LAUNCH_CHECK();
-    INCH_CUDA(cudaMemcpyAsync(&h, w.st, sizeof(State), cudaMemcpyDeviceToHost, stream));
+  k_init<<<bl, 256, 0, stream>>>(seed_order, n, w.order, w.claim, w.par, w.rank, w.ctl);
+  INCH_LAUNCH_CHECK();
+  k_join_few<<<bl, 256, 0, stream>>>(rowptr, cols, n, w.rank, w.par, w.ctl);
+  INCH_LAUNCH_CHECK();
+  k_flatten<<<bl, 256, 0, stream>>>(n, w.par, w.ctl);
+  INCH_LAUNCH_CHECK();
+  k_join_all<<<bw, 256, 0, stream>>>(rowptr, cols, n, w.rank, w.par, w.ctl);
+  INCH_LAUNCH_CHECK();
+  k_flatten<<<bl, 256, 0, stream>>>(n, w.par, w.ctl);
+  INCH_LAUNCH_CHECK();
+  k_roots<<<grid_for(n + 1, 256, 148 * 16), 256, 0, stream>>>(seed_order, n, w.par, w.cnt, w.ctl);
+  INCH_LAUNCH_CHECK();
+  size_t cb = w.cub_bytes;
+  INCH_CUDA(cub::DeviceScan::ExclusiveSum(w.cub_tmp, cb, w.cnt, w.cidx, (int)(n + 1), stream));
+  k_seed<<<bl, 256, 0, stream>>>(seed_order, n, w.cidx, w.order, w.claim, w.ctl);
+  INCH_LAUNCH_CHECK();
+
+  Ctl h{};
+  int comps = 0;
+  const int* count = w.cidx + n;
+  for (int all = 1; all >= 0; --all) {
+    if (all == 0) {
+      INCH_CUDA(cudaMemsetAsync(w.ctl, 0, sizeof(Ctl), stream));
+      k_init<<<bl, 256, 0, stream>>>(seed_order, n, w.order, w.claim, w.par, w.rank, w.ctl);
+      INCH_LAUNCH_CHECK();
+    }
+    void* args[] = {&rowptr, &cols, &degree, &seed_order, &w.par, &count, &n, &w.order, &w.claim, &w.cnt,
+                    &w.blocksum, &w.ctl, &all};
+    INCH_CUDA(cudaLaunchCooperativeKernel((const void*)k_bfs, dim3(blocks), dim3(kWarps * 32), args, kSmem, stream));
+    INCH_CUDA(cudaMemcpyAsync(&h, w.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, stream));
+    if (all) INCH_CUDA(cudaMemcpyAsync(&comps, count, sizeof(int), cudaMemcpyDeviceToHost, stream));
     INCH_CUDA(cudaStreamSynchronize(stream));
-    ++levels;
-    INCH_CUDA(cudaMemcpyAsync(&bad, w.flag, sizeof(int), cudaMemcpyDeviceToHost, stream));
-    INCH_CUDA(cudaStreamSynchronize(stream));
-    INCH_REQUIRE(bad == 0, INCH_INVALID_ARG, "inch_rcm: adjacency lists contain duplicates");
-    INCH_REQUIRE(h.n <= n && levels <= n + 1, INCH_INVALID_ARG, "inch_rcm: inconsistent adjacency (not symmetric?)");
+    INCH_REQUIRE(h.bad != 1, INCH_INVALID_ARG, "inch_rcm: seed_order is not a permutation of 0..n-1");
+    INCH_REQUIRE(h.bad != 2, INCH_LIMIT, "inch_rcm: a row has more than %d neighbours", kCap);
+    INCH_REQUIRE(h.bad == 0, INCH_INVALID_ARG, "inch_rcm: column index out of range");
+    INCH_REQUIRE(h.flag != kTimeout, INCH_TIMEOUT, "inch_rcm: the blocks of the search lost each other");
+    INCH_REQUIRE(h.flag == 0 && h.visited <= n, INCH_INVALID_ARG, "inch_rcm: adjacency lists contain duplicates");
+    if (h.visited == n) {
+      if (!all) comps = 1;                  // already in sequential order
+      break;
+    }
   }
-  INCH_REQUIRE(h.n == n, INCH_INVALID_ARG, "inch_rcm: visited %lld of %lld atoms", (long long)h.n, (long long)n);
-  k_finish<<<bl, 256, 0, stream>>>(w.order, n, rcm_order, undo);
+  INCH_REQUIRE(h.visited == n, INCH_INVALID_ARG, "inch_rcm: visited %lld of %lld atoms", (long long)h.visited,
+               (long long)n);
+  const int* order = w.order;
+  if (comps > 1) {
+    k_keys<<<bl, 256, 0, stream>>>(w.order, n, w.par, w.rank, w.cidx, w.key);
+    INCH_LAUNCH_CHECK();
+    int bits = 1;
+    while (bits < 31 && (int64_t(1) << bits) < comps) ++bits;
+    cb = w.cub_bytes;
+    INCH_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, cb, w.key, w.cnt, w.order, w.order2, (int)n, 0, bits, stream));
+    order = w.order2;
+  }
+  k_finish<<<bl, 256, 0, stream>>>(order, n, rcm_order, undo);
   INCH_LAUNCH_CHECK();
-  if (n_levels_host) *n_levels_host = levels;
+  if (n_levels_host) *n_levels_host = h.levels;
   return INCH_OK;
 }
