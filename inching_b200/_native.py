@@ -595,9 +595,6 @@ def spmm_groups_seg(n_atoms, rows_per_group, gptr, gent, diag, X, Y, atom_seg, s
 # ---------------------------------------------------------------------------
 # Message-passing network kernels (learned warm start)
 # ---------------------------------------------------------------------------
-_gemm_ws = {}
-
-
 def mp_gemm(A, B, C, beta=0.0):
     """C = A B + beta C (FP32) with the package's dense-layer kernel; A, B may be any
     strided 2-D views (transposes included), C row-major with unit column stride."""
@@ -610,11 +607,7 @@ def mp_gemm(A, B, C, beta=0.0):
         raise AssertionError("ABORTED. mp_gemm: shapes or output layout do not match")
     L = lib()
     need = L.inch_mp_gemm_workspace_size(M, N, K)
-    dev = C.device.index
-    ws = _gemm_ws.get(dev)
-    if ws is None or ws.numel() < need:
-        ws = _ws(need, C.device)
-        _gemm_ws[dev] = ws
+    ws = _ws(need, C.device)        # this call's own: products may run on several streams at once
     check(L.inch_mp_gemm(M, N, K, _ptr(A), A.stride(0), A.stride(1), _ptr(B), B.stride(0), B.stride(1), _ptr(C),
                          C.stride(0), float(beta), _ptr(ws), ws.numel(), _stream()))
     _count(1 if need <= 256 else 2)
