@@ -84,6 +84,7 @@ class BeadGraph:
         self.ef = torch.stack([d / self.rc_nm, contacts / 64.0, torch.clamp(self.rc_nm / d, max=10.0) / 10.0,
                                torch.ones_like(d)], dim=1).float().contiguous()
         self.x = self.x.contiguous()
+        self.ones = torch.ones((1, max(nb, self.E)), dtype=torch.float32, device=dev)   # left factor of column sums
 
     def _contacts(self, rowptr, cols, nb):
         """Atom-atom contacts (pairs within the atomic cutoff) between each bead pair."""
@@ -128,17 +129,10 @@ def _mm(A, B, out=None, accumulate=False):
     return _native.mp_gemm(A, B, out, 1.0 if accumulate else 0.0)
 
 
-_ones = {}
-
-
-def _colsum(Y, out):
-    """out (1, F) += column sums of Y (rows, F), as ones^T Y on the same kernel."""
-    r = Y.shape[0]
-    o = _ones.get((Y.device, r))
-    if o is None:
-        o = torch.ones((1, r), dtype=torch.float32, device=Y.device)
-        _ones[(Y.device, r)] = o
-    return _native.mp_gemm(o, Y, out, 1.0)
+def _colsum(G, Y, out):
+    """out (1, F) += column sums of Y (rows, F; a row a bead or an edge of G), as ones^T Y
+    on the same kernel."""
+    return _native.mp_gemm(G.ones[:, :Y.shape[0]], Y, out, 1.0)
 
 
 class WarmStartMPNN:
@@ -218,7 +212,7 @@ class WarmStartMPNN:
         ds = torch.empty(G.E, dtype=torch.float32, device=dgamma.device)
         _native.mp("softplus", c["s"], G.E, GAMMA_FLOOR, None, dgamma.contiguous(), ds)
         _mm(c["R"].t(), ds[:, None], out=g["wo"], accumulate=True)
-        _colsum(ds[:, None], g["bo"][None, :])
+        _colsum(G, ds[:, None], g["bo"][None, :])
         dR = (ds[:, None] * p["wo"].reshape(1, -1)).contiguous()
         dh = torch.zeros((G.n, WIDTH), dtype=torch.float32, device=ds.device)
         _native.mp("edge_pair_bwd", dR, G.src, G.dst, G.E, WIDTH, EDGE_F, dh)
@@ -227,7 +221,7 @@ class WarmStartMPNN:
             dT = dh.clone()
             _native.mp("relu_bwd", dT, T, dT.numel())
             _mm(U.t(), dT, out=g[f"Wu{l}"], accumulate=True)
-            _colsum(dT, g[f"bu{l}"][None, :])
+            _colsum(G, dT, g[f"bu{l}"][None, :])
             dU = _mm(dT, p[f"Wu{l}"].t())
             dM = dU[:, WIDTH:].contiguous()
             dh = dh + dU[:, :WIDTH]
@@ -235,13 +229,13 @@ class WarmStartMPNN:
             _native.mp("segment_sum_bwd", dM, G.mp_rowptr, G.dst, G.E, WIDTH, dA)
             _native.mp("relu_bwd", dA, A, dA.numel())
             _mm(Z.t(), dA, out=g[f"Wm{l}"], accumulate=True)
-            _colsum(dA, g[f"bm{l}"][None, :])
+            _colsum(G, dA, g[f"bm{l}"][None, :])
             dZ = _mm(dA, p[f"Wm{l}"].t())
             dh = dh.contiguous()
             _native.mp("edge_concat_bwd", dZ, G.src, G.E, WIDTH, EDGE_F, dh)
         _native.mp("relu_bwd", dh, c["h0"], dh.numel())
         _mm(G.x.t(), dh, out=g["W0"], accumulate=True)
-        _colsum(dh, g["b0"][None, :])
+        _colsum(G, dh, g["b0"][None, :])
 
     def adam(self, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
         self.step += 1

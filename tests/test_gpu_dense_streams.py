@@ -48,3 +48,18 @@ def test_products_keep_no_memory():
     before = torch.cuda.memory_allocated()
     _native.mp_gemm(A, B, C)
     assert torch.cuda.memory_allocated() == before
+
+
+def test_gradients_keep_no_memory():
+    """A pass over a graph leaves nothing behind once the graph is gone."""
+    from inching_b200 import synth
+    from inching_b200.learned import BeadGraph, WarmStartMPNN
+    model = WarmStartMPNN(seed=1)
+    held = []
+    for atoms in (800, 1400, 2000):
+        G = BeadGraph(torch.from_numpy(synth.globule(atoms, seed=2) / 10.0).cuda())
+        gamma, c = model.forward(G)
+        model.backward(G, c, torch.ones_like(gamma))
+        del G, gamma, c
+        held.append(torch.cuda.memory_allocated())
+    assert held[0] == held[1] == held[2]
