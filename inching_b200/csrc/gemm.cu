@@ -5,9 +5,10 @@
 // FP32 FMAs bound the layers (2 * 132 * 128 flops for 1 KB of an edge's row), so the
 // main kernel is a register-tiled one: 128 x 128 outputs a block, 8 x 8 a thread as
 // packed f32x2 FMAs, 16 steps of K staged at a time through registers into the other
-// of two shared buffers.  Every output sums its terms in the order of K with one
-// rounding a term, whatever the tile, so the choice of kernel does not change the bits
-// of an unsplit product.  Forward and backward pass on the bead graph of the 100k-atom assembly:
+// of two shared buffers.  Up to K = 2,048 every output sums its terms in the order of K
+// with one rounding a term, whatever the tile, so the choice of kernel does not change
+// the bits (beyond it K may be split, and the skinny kernel sums 8 interleaved parts of
+// K).  Forward and backward pass on the bead graph of the 100k-atom assembly:
 // 16.8 ms with 64 x 64 tiles of 4 x 4 outputs a thread, staged element by element, for
 // every product (14.5 ms of it in them), 5.7 ms with these kernels (3.4 ms).
 //
@@ -24,6 +25,7 @@ namespace {
 
 constexpr int kBN = 128, kBK = 16;
 constexpr int kSkinny = 8;           // most rows of the skinny kernel
+constexpr int kLongK = 2048;         // K beyond which K is split and few rows or columns are skinny
 
 struct Gemm {
   int M, N, K;
@@ -336,7 +338,7 @@ int cdiv(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 // K splits of a product with `tiles` output tiles: two blocks an SM, at least 256 steps
 // of K each; none where the output fills the SMs or K is short.
 int splits_for(int64_t tiles, int K) {
-  if (tiles >= 148 || K <= 2048) return 1;
+  if (tiles >= 148 || K <= kLongK) return 1;
   int sp = cdiv(2 * 148, tiles);
   const int by_k = cdiv(K, 256);
   if (sp > by_k) sp = by_k;
@@ -375,7 +377,7 @@ extern "C" size_t inch_mp_gemm_workspace_size(int32_t M, int32_t N, int32_t K) {
   if (M < 1 || N < 1 || K < 1) return 256;
   const int sp = most_splits(M, N, K);
   // the skinny kernel leaves its one part in the workspace too
-  const bool narrow = M <= kSkinny || N <= kSkinny;
+  const bool narrow = (M <= kSkinny || N <= kSkinny) && K > kLongK;
   size_t need = sp > 1 || narrow ? (size_t)sp * M * N * sizeof(float) + 256 : 256;
   if (M > 128 && M % 128 != 0 && M % 128 <= kSkinny) {     // whole tiles and the rest apart
     const size_t whole = inch_mp_gemm_workspace_size(M / 128 * 128, N, K);
@@ -396,8 +398,8 @@ extern "C" inch_status inch_mp_gemm(int32_t M, int32_t N, int32_t K, const float
   float* part = ws != nullptr && ws_bytes >= inch_mp_gemm_workspace_size(M, N, K) ? static_cast<float*>(ws) : nullptr;
   const auto al16 = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
   // skinny products over a long K: the long operand's unit stride lies along the output
-  const bool few_rows = M <= kSkinny && sbn == 1 && K > 2048;
-  const bool few_cols = N <= kSkinny && sai == 1 && K > 2048 && !few_rows;
+  const bool few_rows = M <= kSkinny && sbn == 1 && K > kLongK;
+  const bool few_cols = N <= kSkinny && sai == 1 && K > kLongK && !few_rows;
   if ((few_rows || few_cols) && part != nullptr) {
     const int n = few_rows ? N : M;
     const float* L = few_rows ? B : A;
@@ -411,7 +413,7 @@ extern "C" inch_status inch_mp_gemm(int32_t M, int32_t N, int32_t K, const float
     return INCH_OK;
   }
   Gemm g{M, N, K, A, sai, sak, B, sbk, sbn, C, ldc, beta, K, nullptr};
-  if (N == 1 && K <= 2048) {
+  if (N == 1 && K <= kLongK) {
     k_gemv<<<grid_for(M, 128, 148 * 16), 128, 0, s>>>(g, sak == 1 && sai % 4 == 0 && K % 4 == 0 && al16(A));
     INCH_LAUNCH_CHECK();
     return INCH_OK;
@@ -421,14 +423,14 @@ extern "C" inch_status inch_mp_gemm(int32_t M, int32_t N, int32_t K, const float
   const bool fast = (ak || am) && (bn || bk) && al16(A) && al16(B) && M >= 16 && N >= 16;
   // a few rows beyond whole tiles over a long K (132 = 128 + 4 features by the edges) go
   // to the skinny kernel instead of a second, nearly empty tile
-  if (fast && am && bn && K > 2048 && M > 128 && M % 128 != 0 && M % 128 <= kSkinny && part != nullptr) {
+  if (fast && am && bn && K > kLongK && M > 128 && M % 128 != 0 && M % 128 <= kSkinny && part != nullptr) {
     const int M0 = M / 128 * 128;
     inch_status st = inch_mp_gemm(M0, N, K, A, sai, sak, B, sbk, sbn, C, ldc, beta, ws, ws_bytes, s);
     if (st != INCH_OK) return st;
     return inch_mp_gemm(M - M0, N, K, A + M0, sai, sak, B, sbk, sbn, C + M0 * ldc, ldc, beta, ws, ws_bytes, s);
   }
   // 128-row tiles where they fill the SMs or K is split anyway, else 64-row ones
-  const bool tall = (int64_t)cdiv(M, 128) * cdiv(N, kBN) >= 148 || K > 2048;
+  const bool tall = (int64_t)cdiv(M, 128) * cdiv(N, kBN) >= 148 || K > kLongK;
   const int bm = fast ? (tall ? 128 : 64) : kGM;
   const int mt = cdiv(M, bm), nt = cdiv(N, fast ? kBN : kGN);
   const int sp = splits_for((int64_t)mt * nt, K);
