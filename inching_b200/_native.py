@@ -83,6 +83,7 @@ _SIGS = {
     "inch_hessian_assemble_pbc_xy": (ctypes.c_int, [c_void_p, c_int64, c_double, c_double, c_void_p, c_void_p,
                                                     c_void_p, c_double, c_double, c_void_p, c_void_p, c_void_p,
                                                     c_void_p, c_void_p]),
+    "inch_last_launches": (c_int32, []),
     "inch_rcm_workspace_size": (c_size_t, [c_int64]),
     "inch_rcm": (ctypes.c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p,
                                 POINTER(c_int32), c_void_p, c_size_t, c_void_p]),
@@ -258,7 +259,7 @@ def cuthill_mckee(rowptr, cols, degree, seed_order):
     levels = c_int32(0)
     check(L.inch_rcm(_ptr(rowptr), _ptr(cols), _ptr(degree), _ptr(seed_order), n, _ptr(order), _ptr(undo),
                      ctypes.byref(levels), _ptr(ws), ws.numel(), _stream()))
-    _count(13)
+    _count(L.inch_last_launches())
     return order, undo, levels.value
 
 
@@ -610,7 +611,7 @@ def mp_gemm(A, B, C, beta=0.0):
     ws = _ws(need, C.device)        # this call's own: products may run on several streams at once
     check(L.inch_mp_gemm(M, N, K, _ptr(A), A.stride(0), A.stride(1), _ptr(B), B.stride(0), B.stride(1), _ptr(C),
                          C.stride(0), float(beta), _ptr(ws), ws.numel(), _stream()))
-    _count(1 if need <= 256 else 2)
+    _count(L.inch_last_launches())
     return C
 
 

@@ -21,6 +21,9 @@
 #include "common.cuh"
 
 namespace inch {
+
+thread_local int last_launches = 0;  // of the calling thread's last product or order
+
 namespace {
 
 constexpr int kBN = 128, kBK = 16;
@@ -373,6 +376,8 @@ cudaError_t skinny(int M, int N, int K, const float* S, int64_t sm, int64_t sk, 
 
 using namespace inch;
 
+extern "C" int32_t inch_last_launches(void) { return last_launches; }
+
 extern "C" size_t inch_mp_gemm_workspace_size(int32_t M, int32_t N, int32_t K) {
   if (M < 1 || N < 1 || K < 1) return 256;
   const int sp = most_splits(M, N, K);
@@ -410,12 +415,14 @@ extern "C" inch_status inch_mp_gemm(int32_t M, int32_t N, int32_t K, const float
     const cudaError_t e = few_rows ? run(M, N, K, A, sai, sak, L, ldl, C, ldc, 1, beta, sp, part, s)
                                    : run(N, M, K, B, sbn, sbk, L, ldl, C, 1, ldc, beta, sp, part, s);
     INCH_REQUIRE(e == cudaSuccess, INCH_CUDA_ERROR, "inch_mp_gemm: %s", cudaGetErrorString(e));
+    last_launches = 2;
     return INCH_OK;
   }
   Gemm g{M, N, K, A, sai, sak, B, sbk, sbn, C, ldc, beta, K, nullptr};
   if (N == 1 && K <= kLongK) {
     k_gemv<<<grid_for(M, 128, 148 * 16), 128, 0, s>>>(g, sak == 1 && sai % 4 == 0 && K % 4 == 0 && al16(A));
     INCH_LAUNCH_CHECK();
+    last_launches = 1;
     return INCH_OK;
   }
   const bool ak = sak == 1 && sai % 4 == 0 && K % 4 == 0, am = sai == 1 && sak % 4 == 0 && M % 4 == 0;
@@ -427,7 +434,10 @@ extern "C" inch_status inch_mp_gemm(int32_t M, int32_t N, int32_t K, const float
     const int M0 = M / 128 * 128;
     inch_status st = inch_mp_gemm(M0, N, K, A, sai, sak, B, sbk, sbn, C, ldc, beta, ws, ws_bytes, s);
     if (st != INCH_OK) return st;
-    return inch_mp_gemm(M - M0, N, K, A + M0, sai, sak, B, sbk, sbn, C + M0 * ldc, ldc, beta, ws, ws_bytes, s);
+    const int whole = last_launches;
+    st = inch_mp_gemm(M - M0, N, K, A + M0, sai, sak, B, sbk, sbn, C + M0 * ldc, ldc, beta, ws, ws_bytes, s);
+    last_launches += whole;
+    return st;
   }
   // 128-row tiles where they fill the SMs or K is split anyway, else 64-row ones
   const bool tall = (int64_t)cdiv(M, 128) * cdiv(N, kBN) >= 148 || K > kLongK;
@@ -444,6 +454,7 @@ extern "C" inch_status inch_mp_gemm(int32_t M, int32_t N, int32_t K, const float
   // 1,165 us with the rows first, 1,008 this way; an A of 164 MB is read once).  The other
   // direction is a grid's second dimension, so more tiles than that holds go in several
   // launches (never of a split product).
+  last_launches = 0;
   const int across = fast ? kGridY * kBN : kGridY * kGM;
   for (int64_t at = 0; at < (fast ? N : M); at += across) {
     Gemm h = g;
@@ -469,10 +480,12 @@ extern "C" inch_status inch_mp_gemm(int32_t M, int32_t N, int32_t K, const float
     else TILE(64, false, false);
 #undef TILE
     INCH_LAUNCH_CHECK();
+    ++last_launches;
   }
   if (g.part != nullptr) {
     k_gemm_reduce<<<grid_for((int64_t)M * N, 32, 148 * 8), 256, 0, s>>>(M, N, zs, part, C, ldc, 1, beta);
     INCH_LAUNCH_CHECK();
+    ++last_launches;
   }
   return INCH_OK;
 }

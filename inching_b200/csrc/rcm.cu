@@ -29,6 +29,9 @@
 #include "common.cuh"
 
 namespace inch {
+
+extern thread_local int last_launches;
+
 namespace {
 
 constexpr int kWarps = 16;                  // warps of a BFS block
@@ -481,6 +484,7 @@ extern "C" inch_status inch_rcm(const int64_t* rowptr, const int32_t* cols, cons
   k_seed<<<bl, 256, 0, stream>>>(seed_order, n, w.cidx, w.order, w.claim, w.ctl);
   INCH_LAUNCH_CHECK();
 
+  int launched = 10;                        // so far; a CUB scan or sort counts as one
   Ctl h{};
   int comps = 0;
   const int* count = w.cidx + n;
@@ -489,10 +493,12 @@ extern "C" inch_status inch_rcm(const int64_t* rowptr, const int32_t* cols, cons
       INCH_CUDA(cudaMemsetAsync(w.ctl, 0, sizeof(Ctl), stream));
       k_init<<<bl, 256, 0, stream>>>(seed_order, n, w.order, w.claim, w.par, w.rank, w.ctl);
       INCH_LAUNCH_CHECK();
+      ++launched;
     }
     void* args[] = {&rowptr, &cols, &degree, &seed_order, &w.par, &count, &n, &w.order, &w.claim, &w.cnt,
                     &w.blocksum, &w.ctl, &all};
     INCH_CUDA(cudaLaunchCooperativeKernel((const void*)k_bfs, dim3(blocks), dim3(kWarps * 32), args, kSmem, stream));
+    ++launched;
     INCH_CUDA(cudaMemcpyAsync(&h, w.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, stream));
     if (all) INCH_CUDA(cudaMemcpyAsync(&comps, count, sizeof(int), cudaMemcpyDeviceToHost, stream));
     INCH_CUDA(cudaStreamSynchronize(stream));
@@ -517,9 +523,11 @@ extern "C" inch_status inch_rcm(const int64_t* rowptr, const int32_t* cols, cons
     cb = w.cub_bytes;
     INCH_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, cb, w.key, w.cnt, w.order, w.order2, (int)n, 0, bits, stream));
     order = w.order2;
+    launched += 2;
   }
   k_finish<<<bl, 256, 0, stream>>>(order, n, rcm_order, undo);
   INCH_LAUNCH_CHECK();
+  last_launches = launched + 1;
   if (n_levels_host) *n_levels_host = h.levels;
   return INCH_OK;
 }

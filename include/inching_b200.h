@@ -123,6 +123,9 @@ inch_status inch_neighbors_fill_pbc_xy(const double* X_dev, const inch_cell_grid
  * Synchronises once per BFS level.
  * ------------------------------------------------------------------------- */
 size_t inch_rcm_workspace_size(int64_t n_atoms);
+/* Kernels that the calling thread's last inch_rcm or inch_mp_gemm enqueued (a CUB scan
+ * or sort counts as one): both choose their kernels from the inputs. */
+int32_t inch_last_launches(void);
 inch_status inch_rcm(const int64_t* rowptr_dev, const int32_t* cols_dev, const int32_t* degree_dev,
                      const int64_t* seed_order_dev, int64_t n_atoms,
                      int64_t* rcm_order_dev, int64_t* undo_dev, int32_t* n_levels_host,
