@@ -452,9 +452,11 @@ extern "C" inch_status inch_rcm(const int64_t* rowptr, const int32_t* cols, cons
   INCH_CUDA(cudaFuncSetAttribute(k_bfs, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
   INCH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bfs, kWarps * 32, kSmem));
   INCH_REQUIRE(per_sm >= 1, INCH_CUDA_ERROR, "inch_rcm: the BFS kernel does not fit on an SM");
-  // one block per SM while a block's piece of all atoms is short (fewer blocks to
-  // wait for at a barrier), two where the frontiers are wide
-  const int64_t want = n > 200000 ? 2 : 1;
+  // One block per SM for small inputs (fewer blocks to wait for at a barrier: 2,000-atom
+  // path 17.3 ms, with two 17.6), two where a level's rows outnumber a block's warps:
+  // globules of 20,000 / 100,000 / 400,000 atoms 358 / 677 / 1,976 us with one,
+  // 338 / 543 / 1,350 with two; 100,000 atoms at 15 A (800 neighbours) 2,121 and 1,596.
+  const int64_t want = n > 10000 ? 2 : 1;
   const int blocks = static_cast<int>(std::min<int64_t>(std::min<int64_t>(want, per_sm) * sms, kMaxBlocks));
   const int bl = grid_for(n, 256, 148 * 16), bw = grid_for(n, 8, 148 * 16);
 
