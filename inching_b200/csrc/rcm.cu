@@ -240,18 +240,21 @@ k_bfs(const int64_t* __restrict__ rowptr, const int* __restrict__ cols, const in
   for (;;) {
     if (ls == le) {
       if (all || le >= n) break;
-      // the first seed that no earlier component reached
-      if (blockIdx.x == 0 && w == 0) {
+      // The first seed that no earlier component reached: the whole first block looks,
+      // 512 seeds at a time, because the other blocks' wait is bounded (one warp would
+      // pass 10^8 seeds in about their limit).
+      if (blockIdx.x == 0) {
         int64_t p = ctl->seedptr;
-        for (; p < n; p += 32) {
-          const bool open = p + lane < n && __ldcg(claim + seed_order[p + lane]) == kUnset;
+        for (; p < n; p += kWarps * 32) {
+          const int64_t q = p + threadIdx.x;
+          const bool open = q < n && __ldcg(claim + seed_order[q]) == kUnset;
           const unsigned b = __ballot_sync(0xffffffffu, open);
-          if (b != 0) {
-            p += __ffs(b) - 1;
-            break;
-          }
+          if (lane == 0) s_tot[w] = b != 0 ? q + __ffs(b) - 1 : n;
+          if (__syncthreads_or(open)) break;
         }
-        if (lane == 0 && p < n) {
+        if (threadIdx.x == 0 && p < n) {
+          for (int k = kWarps - 1; k >= 0; --k)
+            if (s_tot[k] < n) p = s_tot[k];
           const int sd = static_cast<int>(seed_order[p]);
           order[le] = sd;
           claim[sd] = -1;

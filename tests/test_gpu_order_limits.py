@@ -88,3 +88,16 @@ def test_seeds_not_a_permutation():
     seeds[7] = seeds[8]
     with pytest.raises(AssertionError, match="permutation"):
         _order(rowptr, cols, degree, seeds)
+
+
+def test_seed_behind_many_visited_ones():
+    """Directed lists: the first seed reaches all atoms but the last one in seed order."""
+    n = 5000
+    heads = np.concatenate([np.arange(n - 2), [n - 1]])
+    tails = np.concatenate([np.arange(1, n - 1), [0]])
+    e = np.concatenate([np.stack([heads, tails], 1), np.stack([np.arange(n)] * 2, 1)])
+    e = e[np.lexsort((e[:, 1], e[:, 0]))]
+    rowptr = np.concatenate([[0], np.cumsum(np.bincount(e[:, 0], minlength=n))])
+    degree = np.diff(rowptr)
+    order, _, levels = _order(rowptr, e[:, 1].copy(), degree, np.arange(n))
+    assert np.array_equal(order.cpu().numpy(), np.arange(n)[::-1]) and levels == n
