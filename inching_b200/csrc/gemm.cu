@@ -170,7 +170,9 @@ __global__ void __launch_bounds__(256, 2) k_gemm_tile(Gemm g) {
   }
 }
 
-// Any strides: 64 x 64 tiles staged element by element.
+// Any strides: 64 x 64 tiles staged element by element.  A chunk's eight loads a thread
+// bound it on few tiles (12 x 12 over K = 1,000: 107 us as loops, one load after another;
+// 55 unrolled, all in flight).
 constexpr int kGM = 64, kGN = 64;
 __global__ void __launch_bounds__(256) k_gemm_any(Gemm g) {
   __shared__ float As[kBK][kGM + 4];
@@ -186,12 +188,16 @@ __global__ void __launch_bounds__(256) k_gemm_any(Gemm g) {
     for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
   for (int k0 = k_beg; k0 < k_end; k0 += kBK) {
     // consecutive threads along whichever index is unit-stride
-    for (int t = threadIdx.x; t < kGM * kBK; t += 256) {
+#pragma unroll
+    for (int i = 0; i < kGM * kBK / 256; ++i) {
+      const int t = threadIdx.x + i * 256;
       const int mm = g.sak == 1 ? t / kBK : t % kGM, kk = g.sak == 1 ? t % kBK : t / kGM;
       const int gi = bm + mm, gk = k0 + kk;
       As[kk][mm] = gi < g.M && gk < k_end ? g.A[gi * g.sai + gk * g.sak] : 0.f;
     }
-    for (int t = threadIdx.x; t < kGN * kBK; t += 256) {
+#pragma unroll
+    for (int i = 0; i < kGN * kBK / 256; ++i) {
+      const int t = threadIdx.x + i * 256;
       const int nn = g.sbn == 1 ? t % kGN : t / kBK, kk = g.sbn == 1 ? t / kGN : t % kBK;
       const int gj = bn + nn, gk = k0 + kk;
       Bs[kk][nn] = gj < g.N && gk < k_end ? g.B[gk * g.sbk + gj * g.sbn] : 0.f;
@@ -427,7 +433,16 @@ extern "C" inch_status inch_mp_gemm(int32_t M, int32_t N, int32_t K, const float
   }
   const bool ak = sak == 1 && sai % 4 == 0 && K % 4 == 0, am = sai == 1 && sak % 4 == 0 && M % 4 == 0;
   const bool bn = sbn == 1 && sbk % 4 == 0 && N % 4 == 0, bk = sbk == 1 && sbn % 4 == 0 && K % 4 == 0;
-  const bool fast = (ak || am) && (bn || bk) && al16(A) && al16(B) && M >= 16 && N >= 16;
+  // Register tiles pay where K is long enough to hide their prologue and epilogue and the
+  // tiles are full.  Where its own tiles fill the SMs the general kernel is faster on a
+  // short K (20,000 x 128: K = 4, 7.3 us against 10.2; K = 32, 11.0 both), and up to 64
+  // rows or columns on a middling one (20,000 x 16: K = 16, 4.9 and 6.9; K = 256, 36 and
+  // 46).  Up to 32 rows stay with the tiles (16 x 100,000, K = 4: 12.1 general, 7.6).
+  // Below 16 rows or columns the tiles are mostly padding.
+  const int narrow = std::min(M, N);
+  const bool shallow = M > 32 && (int64_t)cdiv(M, kGM) * cdiv(N, kGN) >= 200 &&
+                       (narrow <= 64 ? K <= 256 : (int64_t)K * cdiv(narrow, 64) <= 48);
+  const bool fast = (ak || am) && (bn || bk) && al16(A) && al16(B) && narrow >= 16 && !shallow;
   // a few rows beyond whole tiles over a long K (132 = 128 + 4 features by the edges) go
   // to the skinny kernel instead of a second, nearly empty tile
   if (fast && am && bn && K > kLongK && M > 128 && M % 128 != 0 && M % 128 <= kSkinny && part != nullptr) {
@@ -439,8 +454,10 @@ extern "C" inch_status inch_mp_gemm(int32_t M, int32_t N, int32_t K, const float
     last_launches += whole;
     return st;
   }
-  // 128-row tiles where they fill the SMs or K is split anyway, else 64-row ones
-  const bool tall = (int64_t)cdiv(M, 128) * cdiv(N, kBN) >= 148 || K > kLongK;
+  // 128-row tiles where they fill the SMs or K is split anyway, else 64-row ones; these too
+  // where half of a 128 x 128 tile would be padding (20,000 x 16 over K = 1,000: 185 us
+  // with 128 rows, 166 with 64)
+  const bool tall = K > kLongK || (narrow > 64 && (int64_t)cdiv(M, 128) * cdiv(N, kBN) >= 148);
   const int bm = fast ? (tall ? 128 : 64) : kGM;
   const int mt = cdiv(M, bm), nt = cdiv(N, fast ? kBN : kGN);
   const int sp = splits_for((int64_t)mt * nt, K);
@@ -451,7 +468,8 @@ extern "C" inch_status inch_mp_gemm(int32_t M, int32_t N, int32_t K, const float
   const int zs = cdiv(K, g.kchunk);
   // The general kernel walks the column tiles of a row of tiles first, the register tiles
   // the rows of a column of tiles (20,000 x 129 over K = 2,052 through the general kernel:
-  // 1,165 us with the rows first, 1,008 this way; an A of 164 MB is read once).  The other
+  // 1,165 us with the rows first, 1,008 the columns, as an A of 164 MB is read once; with
+  // the staging loads issued together 658).  The other
   // direction is a grid's second dimension, so more tiles than that holds go in several
   // launches (never of a split product).
   last_launches = 0;
