@@ -28,7 +28,10 @@ namespace {
 
 constexpr int kBN = 128, kBK = 16;
 constexpr int kSkinny = 8;           // most rows of the skinny kernel
-constexpr int kLongK = 2048;         // K beyond which K is split and few rows or columns are skinny
+// K beyond which K is split and few rows or columns are skinny.  Splitting would pay below it
+// too (48 x 48: K = 2,048 unsplit 124 us, K = 2,049 split 17), but up to the line
+// a sum keeps the order of K, and its bits.
+constexpr int kLongK = 2048;
 
 struct Gemm {
   int M, N, K;
@@ -469,9 +472,9 @@ extern "C" inch_status inch_mp_gemm(int32_t M, int32_t N, int32_t K, const float
   // The general kernel walks the column tiles of a row of tiles first, the register tiles
   // the rows of a column of tiles (20,000 x 129 over K = 2,052 through the general kernel:
   // 1,165 us with the rows first, 1,008 the columns, as an A of 164 MB is read once; with
-  // the staging loads issued together 658).  The other
-  // direction is a grid's second dimension, so more tiles than that holds go in several
-  // launches (never of a split product).
+  // the staging loads issued together 658).  The other direction is a grid's second
+  // dimension, so more tiles than that holds go in several launches (never of a split
+  // product).
   last_launches = 0;
   const int across = fast ? kGridY * kBN : kGridY * kGM;
   for (int64_t at = 0; at < (fast ? N : M); at += across) {

@@ -18,7 +18,7 @@ Hellmann-Feynman, d mu_t / d gamma_e = (u_e . (v_t[a] - v_t[b]))^2 with the
 bead model's eigenvectors v_t, so no differentiation through the eigensolver is
 needed.  The forward and backward passes are hand-written: graph gathers,
 neighbour means, activations, the eigenvalue gradient and the Adam step are the
-package's CUDA kernels (csrc/mpnn.cu); dense layers are cuBLAS GEMMs.
+package's CUDA kernels (csrc/mpnn.cu), the dense layers too (csrc/gemm.cu).
 
 The prolonged block goes through a residual test against random columns (one
 Rayleigh-Ritz each on the fine Hessian, over the leading 64 columns): if its

@@ -120,7 +120,11 @@ inch_status inch_neighbors_fill_pbc_xy(const double* X_dev, const inch_cell_grid
  * unvisited atom in that order seeds each connected component.
  * Outputs the REVERSED order (rcm_order_dev, int64 N) and its inverse
  * (undo_dev, int64 N), as X_KdCuthillMckeeOrder(..., Reverse=True) returns.
- * Synchronises once per BFS level.
+ * One cooperative launch walks all levels.  Synchronises once, and once more for
+ * directed lists (j under i, not i under j) whose components their first seed does
+ * not reach.  INCH_INVALID_ARG: seeds that are no permutation, columns out of range,
+ * rows that list an atom twice; INCH_LIMIT: a row of more than INCH_MAX_DEGREE;
+ * INCH_TIMEOUT: the launch's blocks waited seconds for one another.
  * ------------------------------------------------------------------------- */
 size_t inch_rcm_workspace_size(int64_t n_atoms);
 /* Kernels that the calling thread's last inch_rcm or inch_mp_gemm enqueued (a CUB scan
@@ -189,7 +193,7 @@ inch_status inch_hessian_assemble_pbc_xy(const double* X_dev, int64_t n_atoms, d
 /* ---------------------------------------------------------------------------
  * Message-passing network kernels of the learned warm start (no reference
  * counterpart).  Directed bead-graph edges in CSR by destination: rowptr (N+1),
- * src[e] / dst[e] per edge.  Dense layers are GEMMs done by the caller.
+ * src[e] / dst[e] per edge.
  *   edge_concat      Z[e] = [H[src[e]], EF[e]]           (+ bwd: scatter-add)
  *   segment_sum      M[i] = mean of A over the edges of row i (+ bwd: gather / deg)
  *   bias_relu        Y = relu(Y + b);  relu_bwd  dY *= (Y > 0)
@@ -224,8 +228,10 @@ inch_status inch_mp_adam(float* w, const float* g, float* m1, float* m2, int64_t
 /* The network's dense layers: C = A B + beta C in FP32, with element (i, k) of A at
  * A[i*sai + k*sak] and (k, j) of B at B[k*sbk + j*sbn] (so transposed operands are
  * strides), C row-major with leading dimension ldc.  A product with a small output
- * and a long K splits K into partial tiles added in a fixed order (deterministic);
- * ws: inch_mp_gemm_workspace_size(M, N, K) bytes.  No reference counterpart. */
+ * and a K above 2,048 splits K into partial tiles added in a fixed order
+ * (deterministic); up to there an output's terms are added in the order of K.
+ * ws: inch_mp_gemm_workspace_size(M, N, K) bytes of this call's own until its kernels
+ * are done.  No reference counterpart. */
 size_t inch_mp_gemm_workspace_size(int32_t M, int32_t N, int32_t K);
 inch_status inch_mp_gemm(int32_t M, int32_t N, int32_t K, const float* A, int64_t sai, int64_t sak,
                          const float* B, int64_t sbk, int64_t sbn, float* C, int64_t ldc, float beta,
