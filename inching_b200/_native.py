@@ -87,6 +87,8 @@ _SIGS = {
     "inch_rcm_workspace_size": (c_size_t, [c_int64]),
     "inch_rcm": (ctypes.c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p,
                                 POINTER(c_int32), c_void_p, c_size_t, c_void_p]),
+    "inch_rcm_bounded": (ctypes.c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p,
+                                        POINTER(c_int32), ctypes.c_uint32, c_void_p, c_size_t, c_void_p]),
     "inch_band_slices_workspace_size": (c_size_t, [c_int64, c_int64]),
     "inch_band_slices": (ctypes.c_int, [c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_int64, c_int32,
                                         c_void_p, c_void_p, c_void_p, POINTER(c_int64), c_void_p, c_size_t,

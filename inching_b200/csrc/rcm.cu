@@ -207,7 +207,7 @@ __global__ void k_finish(const int* __restrict__ order, int64_t n, int64_t* __re
 // ---------------------------------------------------------------------------
 // Grid barrier of a cooperative launch (every block resident).  The wait is bounded:
 // a block whose wait runs out records it and leaves, and so do the others.
-__device__ bool grid_barrier(Ctl* ctl, unsigned& target) {
+__device__ bool grid_barrier(Ctl* ctl, unsigned& target, unsigned max_polls) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -217,7 +217,7 @@ __device__ bool grid_barrier(Ctl* ctl, unsigned& target) {
     int ok = 1;
     const volatile unsigned* at = &ctl->arrive;
     for (unsigned polls = 0; static_cast<int>(*at - target) < 0; ++polls)
-      if (polls > kBarrierPolls || ((polls & 1023) == 1023 && *(volatile int*)&ctl->flag == kTimeout)) {
+      if (polls > max_polls || ((polls & 1023) == 1023 && *(volatile int*)&ctl->flag == kTimeout)) {
         atomicExch(&ctl->flag, kTimeout);
         ok = 0;
         break;
@@ -234,7 +234,8 @@ __device__ bool grid_barrier(Ctl* ctl, unsigned& target) {
 __global__ void __launch_bounds__(kWarps * 32, 2)
 k_bfs(const int64_t* __restrict__ rowptr, const int* __restrict__ cols, const int* __restrict__ degree,
       const int64_t* __restrict__ seed_order, const int* __restrict__ par, const int* __restrict__ comp_count,
-      int64_t n, int* order, int* claim, int* cnt, int* blocksum, Ctl* ctl, int all) {
+      int64_t n, int* order, int* claim, int* cnt, int* blocksum, Ctl* ctl, int all,
+      unsigned max_polls) {
   extern __shared__ int s_buf[];            // kCap per warp
   __shared__ int64_t s_pre[kWarps], s_tot[kWarps];
   if (ctl->bad) return;                     // set by earlier kernels only: the same for every block
@@ -267,7 +268,7 @@ k_bfs(const int64_t* __restrict__ rowptr, const int* __restrict__ cols, const in
           ctl->seedptr = p + 1;
         }
       }
-      if (!grid_barrier(ctl, target)) break;
+      if (!grid_barrier(ctl, target, max_polls)) break;
       le = ls + 1;
     }
     const int64_t L = le - ls;
@@ -284,7 +285,7 @@ k_bfs(const int64_t* __restrict__ rowptr, const int* __restrict__ cols, const in
         if (__ldcg(claim + j) > static_cast<int>(q)) atomicMin(claim + j, static_cast<int>(q));
       }
     }
-    if (!grid_barrier(ctl, target)) break;
+    if (!grid_barrier(ctl, target, max_polls)) break;
     // count the children of each q, prefix sums within the block's piece
     for (int64_t q = q0 + w; q < q1; q += kWarps) {
       const int i = __ldcg(order + q);
@@ -323,7 +324,7 @@ k_bfs(const int64_t* __restrict__ rowptr, const int* __restrict__ cols, const in
       }
       if (lane == 0) blocksum[blockIdx.x] = run;
     }
-    if (!grid_barrier(ctl, target)) break;
+    if (!grid_barrier(ctl, target, max_polls)) break;
     int64_t pre = 0, tot = 0;
     for (int b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
       const int v = __ldcg(blocksum + b);
@@ -381,7 +382,7 @@ k_bfs(const int64_t* __restrict__ rowptr, const int* __restrict__ cols, const in
     ls = le;
     le += tot;
     if (le > n) break;                      // the same in every block
-    if (!grid_barrier(ctl, target)) break;
+    if (!grid_barrier(ctl, target, max_polls)) break;
   }
   levels = warp_sum(levels);                // lane 0 of each warp counted
   if (lane == 0 && levels != 0) atomicAdd(&ctl->levels, levels);
@@ -447,6 +448,14 @@ extern "C" size_t inch_rcm_workspace_size(int64_t n) {
 extern "C" inch_status inch_rcm(const int64_t* rowptr, const int32_t* cols, const int32_t* degree,
                                 const int64_t* seed_order, int64_t n, int64_t* rcm_order, int64_t* undo,
                                 int32_t* n_levels_host, void* ws, size_t ws_bytes, cudaStream_t stream) {
+  return inch_rcm_bounded(rowptr, cols, degree, seed_order, n, rcm_order, undo, n_levels_host, kBarrierPolls, ws,
+                          ws_bytes, stream);
+}
+
+extern "C" inch_status inch_rcm_bounded(const int64_t* rowptr, const int32_t* cols, const int32_t* degree,
+                                        const int64_t* seed_order, int64_t n, int64_t* rcm_order, int64_t* undo,
+                                        int32_t* n_levels_host, uint32_t max_polls, void* ws, size_t ws_bytes,
+                                        cudaStream_t stream) {
   INCH_REQUIRE(rowptr && cols && degree && seed_order && rcm_order && undo, INCH_INVALID_ARG,
                "inch_rcm: NULL argument");
   INCH_REQUIRE(n >= 1 && n < (int64_t(1) << 31), INCH_INVALID_ARG, "inch_rcm: n_atoms out of range");
@@ -507,7 +516,7 @@ extern "C" inch_status inch_rcm(const int64_t* rowptr, const int32_t* cols, cons
       ++launched;
     }
     void* args[] = {&rowptr, &cols, &degree, &seed_order, &w.par, &count, &n, &w.order, &w.claim, &w.cnt,
-                    &w.blocksum, &w.ctl, &all};
+                    &w.blocksum, &w.ctl, &all, &max_polls};
     INCH_CUDA(cudaLaunchCooperativeKernel((const void*)k_bfs, dim3(blocks), dim3(kWarps * 32), args, kSmem, stream));
     ++launched;
     INCH_CUDA(cudaMemcpyAsync(&h, w.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, stream));

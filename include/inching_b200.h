@@ -134,6 +134,12 @@ inch_status inch_rcm(const int64_t* rowptr_dev, const int32_t* cols_dev, const i
                      const int64_t* seed_order_dev, int64_t n_atoms,
                      int64_t* rcm_order_dev, int64_t* undo_dev, int32_t* n_levels_host,
                      void* ws_dev, size_t ws_bytes, cudaStream_t stream);
+/* inch_rcm with the caller's bound on a wait: looks at the grid barrier (about 0.7 us
+ * each) before the search gives up with INCH_TIMEOUT.  The outputs are not written then. */
+inch_status inch_rcm_bounded(const int64_t* rowptr_dev, const int32_t* cols_dev, const int32_t* degree_dev,
+                             const int64_t* seed_order_dev, int64_t n_atoms,
+                             int64_t* rcm_order_dev, int64_t* undo_dev, int32_t* n_levels_host,
+                             uint32_t max_polls, void* ws_dev, size_t ws_bytes, cudaStream_t stream);
 
 /* ---------------------------------------------------------------------------
  * Ungapped band slices of X_KdUngappedMinMaxNeighbor (Fuel/Coordinate/T1.py:371-481)

@@ -101,3 +101,28 @@ def test_seed_behind_many_visited_ones():
     degree = np.diff(rowptr)
     order, _, levels = _order(rowptr, e[:, 1].copy(), degree, np.arange(n))
     assert np.array_equal(order.cpu().numpy(), np.arange(n)[::-1]) and levels == n
+
+
+def test_wait_that_runs_out():
+    """A bound that no block's wait keeps: the call says so, and the next one is answered."""
+    import ctypes
+    n = 2000
+    rowptr, cols = _ladder(n, n)
+    degree = np.diff(rowptr)
+    d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in
+         (rowptr.astype(np.int64), cols.astype(np.int32), degree.astype(np.int32),
+          np.argsort(degree).astype(np.int64))]
+    L = _native.lib()
+    ws = torch.empty(L.inch_rcm_workspace_size(n), dtype=torch.uint8, device="cuda")
+    order, undo = (torch.empty(n, dtype=torch.int64, device="cuda") for _ in range(2))
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+
+    def call(polls):
+        return L.inch_rcm_bounded(*[p(t) for t in d], n, p(order), p(undo), None, polls, p(ws), ws.numel(),
+                                  ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+
+    assert call(0) == _native.INCH_TIMEOUT
+    assert call(1 << 24) == _native.INCH_OK
+    torch.cuda.synchronize()
+    ref, _ = og.cuthill_mckee_c(rowptr, cols, degree, np.argsort(degree))
+    assert np.array_equal(order.cpu().numpy(), ref)
